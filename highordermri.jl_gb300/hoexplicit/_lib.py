@@ -47,6 +47,13 @@ HOE_CG_CONVERGED = 1
 HOE_CG_STOPPED = 2
 
 
+def stored(t):
+    """The tensor with its values in memory as they read: a lazy conjugate
+    (x.conj()) or negation (x.conj().imag) is carried out, since the library gets
+    the address of the values."""
+    return t.resolve_conj().resolve_neg()
+
+
 class ArgumentError(ValueError):
     """Julia ``ArgumentError`` counterpart."""
 

@@ -14,7 +14,7 @@ import ctypes
 import weakref
 
 from . import _lib
-from ._lib import ArgumentError, DimensionMismatch
+from ._lib import ArgumentError, DimensionMismatch, stored
 from .recon import DEFAULT_ITERATIONS, DEFAULT_REL_TOL, STATUS, _device_vector
 
 
@@ -57,7 +57,7 @@ class OperatorBatch:
                 v = torch.from_numpy(v)
             if v.numel() != n:
                 raise DimensionMismatch(f"{name} has length {v.numel()}, expected {n}")
-            out.append(v.to(device=op.torch_device, dtype=torch.complex64).reshape(-1).contiguous())
+            out.append(stored(v.to(device=op.torch_device, dtype=torch.complex64).reshape(-1)).contiguous())
         return out
 
     def info(self) -> dict:
@@ -87,7 +87,8 @@ class OperatorBatch:
         import torch
         x = self._vecs(xs, [op.ncol for op in self.ops], "x")
         out = [torch.empty(op.ncol, dtype=torch.complex64, device=op.torch_device) for op in self.ops]
-        d = None if D is None else _ptrs(list(D))
+        D = None if D is None else [None if v is None else stored(v) for v in D]
+        d = None if D is None else _ptrs(D)
         _lib.check(_lib.load().hoe_batch_normal(self._batch(), d, _ptrs(x), _ptrs(out), self._stream()),
                    batch=self._b)
         return out
@@ -105,6 +106,10 @@ class OperatorBatch:
                  for op, v in zip(self.ops, weights)]
         if out is None:
             out = [torch.empty(op.ncol, dtype=torch.complex64, device=op.torch_device) for op in self.ops]
+        elif any(v.is_conj() or v.is_neg() for v in out):
+            xs, info = self.recon(datas, weights, iterations=iterations, rel_tol=rel_tol, lam=lam,
+                                  use_graph=use_graph, stats=stats)
+            return [v.copy_(x.view_as(v)) for v, x in zip(out, xs)], info
         p = _lib.HoeCgParams(int(iterations), int(bool(use_graph)), float(rel_tol), float(lam))
         st = (_lib.HoeCgStats * len(self.ops))()
         _lib.check(_lib.load().hoe_batch_recon(self._batch(), _ptrs(d), _ptrs(w), _ptrs(out), ctypes.byref(p),

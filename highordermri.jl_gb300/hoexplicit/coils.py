@@ -14,7 +14,7 @@ from dataclasses import dataclass
 import numpy as np
 
 from . import _lib
-from ._lib import ArgumentError, DimensionMismatch
+from ._lib import ArgumentError, DimensionMismatch, stored
 
 
 def _torch():
@@ -68,7 +68,7 @@ def _coil_last(array, coil_dim):
 
 def _device_colmajor(mat, dtype):
     torch = _torch()
-    return mat.to(device="cuda", dtype=dtype).t().contiguous().reshape(-1)
+    return stored(mat.to(device="cuda", dtype=dtype).t().contiguous().reshape(-1))
 
 
 def estimate_noise_covariance(noise_data, *, coil_dim: int = -1, center: bool = True) -> np.ndarray:

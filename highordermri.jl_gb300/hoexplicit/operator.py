@@ -26,7 +26,7 @@ import weakref
 import numpy as np
 
 from . import _lib
-from ._lib import ArgumentError, DimensionMismatch
+from ._lib import ArgumentError, DimensionMismatch, stored
 from .model import Grid, basisfunc_spha, prep_concomitant, prep_kspha
 
 ENGINES = {"fp32": _lib.HOE_ENGINE_FP32_SIMT, "simt": _lib.HOE_ENGINE_FP32_SIMT,
@@ -77,7 +77,7 @@ class _Vec:
             raise ArgumentError(f"{name} is on cuda:{v.device.index}, operator on cuda:{op.device}")
         if v.dtype != torch.complex64:
             v = v.to(torch.complex64)
-        self.t = v.reshape(-1).contiguous()
+        self.t = stored(v.reshape(-1)).contiguous()
 
     def out_like(self, result):
         if self.host == "numpy":
@@ -93,13 +93,13 @@ class _Vec:
 
 def _direct(op, v, n):
     """Whether v can go to the library as it is: n contiguous complex64 values
-    on the operator's GPU, what _Vec would make of it.  Small products are bound
+    on the operator's GPU as they read, what _Vec would make of it.  Small products are bound
     by the host: with _Vec and the stream object a forward and an adjoint at
     64x64 / 4,096 samples / 8 coils took 40 us to queue, without 20, and the GPU
     needs 36."""
     torch = _torch()
     return (type(v) is torch.Tensor and v.dtype is torch.complex64 and v.is_cuda and v.numel() == n
-            and v.get_device() == op.device and v.is_contiguous())
+            and v.get_device() == op.device and v.is_contiguous() and not v.is_conj() and not v.is_neg())
 
 
 # The tensor-core engine's execution plans (hoe_desc.tc_plan, hoe_autotune);
@@ -340,9 +340,10 @@ class ExplicitGB300Op:
     # ------------------------------------------------------------ products
     def _io(self, t, n, name, role, torch, stream):
         """Device view of an in-place product operand.  A CUDA tensor is used
-        as is; a host tensor goes through a device buffer that the operator
-        keeps per (stream, role, length), reused in stream order.  Returns
-        (device tensor, host tensor to copy the result into or None, pinned)."""
+        as is, a lazily conjugated or negated one through a plain one of the call; a
+        host tensor goes through a device buffer that the operator keeps per (stream,
+        role, length), reused in stream order.  Returns (device tensor, tensor to
+        copy the operand from or the result into or None, whether without waiting)."""
         if not isinstance(t, torch.Tensor) or t.dtype != torch.complex64 or not t.is_contiguous():
             raise ArgumentError(f"{name} must be a contiguous complex64 torch tensor")
         if t.numel() != n:
@@ -350,6 +351,8 @@ class ExplicitGB300Op:
         if t.is_cuda:
             if t.get_device() != self.device:
                 raise ArgumentError(f"{name} is on cuda:{t.get_device()}, operator on cuda:{self.device}")
+            if t.is_conj() or t.is_neg():
+                return torch.empty(n, dtype=torch.complex64, device=self.torch_device), t.detach().view(-1), True
             return t, None, False
         key = (stream, role, n)
         buf = self._stage.get(key)
@@ -521,6 +524,9 @@ class NormalOp:
 
     def prod_(self, out, x):
         op = self.op
+        x = stored(x)
+        if out.is_conj() or out.is_neg():
+            return out.copy_(self.prod_(stored(out.detach()), x))
         _lib.check(_lib.load().hoe_normal(op._handle(), self.D.data_ptr(), x.data_ptr(),
                                           out.data_ptr(), op._stream()), op._h)
         return out

@@ -16,7 +16,7 @@ import ctypes
 import numpy as np
 
 from . import _lib
-from ._lib import ArgumentError, DimensionMismatch
+from ._lib import ArgumentError, DimensionMismatch, stored
 
 # RegularizedLeastSquares CGNR keyword defaults: iterations = 10,
 # relTol = eps of the operator's real type.
@@ -93,7 +93,7 @@ def _device_vector(op, v, rows: int, cols: int, name: str):
             raise DimensionMismatch(f"{name} has shape {tuple(t.shape)}, expected {(rows, cols)}")
         if t.device.type == "cuda" and t.device.index != op.device:
             raise ArgumentError(f"{name} is on cuda:{t.device.index}, operator on cuda:{op.device}")
-        return t.to(device=op.torch_device, dtype=torch.complex64).t().contiguous().reshape(-1)
+        return stored(t.to(device=op.torch_device, dtype=torch.complex64).t().contiguous().reshape(-1))
     raise ArgumentError(f"{name} must be a numpy array or torch tensor")
 
 
@@ -111,6 +111,10 @@ def solve(op, data, weight=None, *, iterations: int = DEFAULT_ITERATIONS, rel_to
         out = torch.empty(op.ncol, dtype=torch.complex64, device=op.torch_device)
     elif out.numel() != op.ncol or out.dtype != torch.complex64 or not out.is_contiguous():
         raise DimensionMismatch("out must be a contiguous complex64 vector of length prod(matrixSize)")
+    elif out.is_conj() or out.is_neg():
+        x, info = solve(op, data, weight, iterations=iterations, rel_tol=rel_tol, lam=lam, use_graph=use_graph,
+                        stats=stats)
+        return out.copy_(x.view_as(out)), info
     p = _lib.HoeCgParams(int(iterations), int(bool(use_graph)), float(rel_tol), float(lam))
     st = _lib.HoeCgStats()
     _lib.check(_lib.load().hoe_recon(h, d.data_ptr(), None if w is None else w.data_ptr(), out.data_ptr(),

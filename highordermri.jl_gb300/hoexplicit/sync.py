@@ -17,7 +17,7 @@ import ctypes
 import numpy as np
 
 from . import _lib
-from ._lib import ArgumentError, DimensionMismatch
+from ._lib import ArgumentError, DimensionMismatch, stored
 from .model import Grid
 from .recon import L2Regularization
 
@@ -39,7 +39,7 @@ def _colmajor(a, name):
     if isinstance(a, torch.Tensor):
         if a.dim() != 2:
             raise DimensionMismatch(f"{name} must be a matrix")
-        return a.to(device="cuda", dtype=torch.float64).t().contiguous().reshape(-1), tuple(a.shape), "torch"
+        return stored(a.to(device="cuda", dtype=torch.float64).t().contiguous().reshape(-1)), tuple(a.shape), "torch"
     raise ArgumentError(f"{name} must be a numpy array or torch tensor")
 
 
@@ -48,7 +48,7 @@ def _vec64(a, name):
     if isinstance(a, np.ndarray):
         return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float64).reshape(-1)).cuda()
     if isinstance(a, torch.Tensor):
-        return a.to(device="cuda", dtype=torch.float64).reshape(-1).contiguous()
+        return stored(a.to(device="cuda", dtype=torch.float64).reshape(-1)).contiguous()
     raise ArgumentError(f"{name} must be a numpy array or torch tensor")
 
 
