@@ -96,6 +96,8 @@ void release_device(hoe_handle *h) {
   hoe::cg_release(h);
   hoe::tc_backward_release(h);
   hoe::tc_release(h);
+  if (h->replanned) cudaEventDestroy(h->replanned);
+  h->replanned = nullptr;
   auto &t = h->t;
   dfree(t.dbeta); dfree(t.kappa); dfree(t.Atab); dfree(t.Btab); dfree(t.csm);
   dfree(t.dbHi); dfree(t.dbLo); dfree(t.kpHi); dfree(t.kpLo);
@@ -998,6 +1000,15 @@ int hoe_set_kspha(hoe_handle *h, const double *kspha, const double *kspha_dt, vo
   if (!kspha) return fail(h, HOE_ERR_ARG, "kspha must be a device pointer");
   DeviceGuard guard(h->device);
   cudaError_t e = hoe::replan_samples(h, kspha, h->t.R0, kspha_dt, h->t.nTerm, nullptr, (cudaStream_t)stream);
+  if (e == cudaSuccess && !h->tc.ready) {
+    // (inside a capture the replays' order is the caller's)
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    e = cudaStreamIsCapturing((cudaStream_t)stream, &capturing);
+    if (e == cudaSuccess && capturing == cudaStreamCaptureStatusNone) {
+      if (!h->replanned) e = cudaEventCreateWithFlags(&h->replanned, cudaEventDisableTiming);
+      if (e == cudaSuccess) e = cudaEventRecord(h->replanned, (cudaStream_t)stream);
+    }
+  }
   return finish(h, e, "hoe_set_kspha");
 }
 

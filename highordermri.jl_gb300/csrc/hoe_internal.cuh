@@ -219,6 +219,9 @@ struct hoe_handle {
   hoe::TcState tc;
   void *tc_host = nullptr;   // tensor-core buffer table (hoe_tc.cu)
   void *tcb_host = nullptr;  // tensor-core backward buffers (hoe_tc_bwd.cu), allocated on first use
+  // the last hoe_set_kspha before the tensor-core engine is prepared: tc_prepare
+  // makes its anchor pairs from the tables which that call's kernels write
+  cudaEvent_t replanned = nullptr;
   hoe::CgState cg;           // device-resident CGNR (hoe_cg.cu)
 };
 

@@ -396,7 +396,9 @@ cudaError_t tc_prepare(hoe_handle *h) {
   // the first forward contraction of this operator stall CTA 0 at stage k
   if (const char *inj = getenv("HOE_INJECT_TC_STALL")) b.injectStall1 = atoi(inj) + 1;
   h->tc_host = new TcBuffers(b);
-  e = anchor_pairs(h, (float2 *)b.AtabP, (float2 *)b.BtabQ, 0);
+  // the tables may still be in the making on another stream
+  e = h->replanned ? cudaEventSynchronize(h->replanned) : cudaSuccess;
+  if (e == cudaSuccess) e = anchor_pairs(h, (float2 *)b.AtabP, (float2 *)b.BtabQ, 0);
   if (e == cudaSuccess) e = cudaStreamSynchronize(0);
   if (e == cudaSuccess && h->tcPlan > 0) e = tc_set_plan(h, h->tcPlan);
   return e;
