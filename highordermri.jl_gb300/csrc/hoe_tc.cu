@@ -653,8 +653,8 @@ cudaError_t tc_derivative_prepare(hoe_handle *h) {
     b.bytesD = bfB + kdB + KF * KF * (sizeof(float) + sizeof(double));
     cudaError_t e = cudaMalloc(&b.memD, b.bytesD);
     if (e != cudaSuccess) { b.memD = nullptr; return e; }
-    b.facCol = (float *)b.memD;
-    b.facRow = (float *)((unsigned char *)b.memD + bfB);
+    b.facCol = (uint16_t *)b.memD;
+    b.facRow = (uint16_t *)((unsigned char *)b.memD + bfB);
     b.Md = (float *)((unsigned char *)b.memD + bfB + kdB);
     h->bytes += (int64_t)b.bytesD;
     // voxel side of the reduced basis: fixed for the operator
@@ -666,7 +666,8 @@ cudaError_t tc_derivative_prepare(hoe_handle *h) {
       cudaFree(b.memD);
       h->bytes -= (int64_t)b.bytesD;
       b.memD = nullptr;
-      b.facCol = b.facRow = b.Md = nullptr;
+      b.facCol = b.facRow = nullptr;
+      b.Md = nullptr;
     }
     return e;
   }

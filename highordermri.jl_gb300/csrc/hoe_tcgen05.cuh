@@ -29,14 +29,14 @@ struct TcBuffers {
   int gridF = 1, gridA = 1, slotsF = 1, slotsA = 1;
   size_t bopFElems = 0, bopAElems = 0, partElems = 0;
   // derivative product (kspha_dt mode), allocated on first use.  Up to 16
-  // coils one pass (fusedD): the factor's TF32 tables facCol and facRow; above, the
+  // coils one pass (fusedD): the factor's BF16 tables facCol and facRow; above, the
   // 128-wide B operand of 64 virtual coils and its partial slots per pass
   uint16_t *bopD = nullptr;
   float2 *partD = nullptr;
-  float *facCol = nullptr;
-  float *facRow = nullptr;
+  uint16_t *facCol = nullptr;
+  uint16_t *facRow = nullptr;
   float *Md = nullptr;      // reduced-basis rotation [KF x KF] of the one-pass path
-  int rankD = 0, kfD = 48;  // its rank and the tables' columns (24, 32 or 48)
+  int rankD = 0, kfD = 48;  // its rank and the tables' 32-bit words a row (24, 32 or 48)
   bool fusedD = false;
   void *memD = nullptr;
   size_t bytesD = 0;
