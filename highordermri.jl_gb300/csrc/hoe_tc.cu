@@ -406,7 +406,10 @@ cudaError_t tc_prepare(hoe_handle *h) {
 
 void tc_release(hoe_handle *h) {
   if (h->tc.buf) cudaFree(h->tc.buf);
-  if (h->tc_host && ((TcBuffers *)h->tc_host)->memD) cudaFree(((TcBuffers *)h->tc_host)->memD);
+  if (const TcBuffers *b = (const TcBuffers *)h->tc_host) {
+    if (b->memM) cudaFree(b->memM);
+    if (b->memD) cudaFree(b->memD);
+  }
   delete (TcBuffers *)h->tc_host;
   h->tc_host = nullptr;
   h->tc = TcState();
@@ -648,24 +651,30 @@ cudaError_t tc_derivative_prepare(hoe_handle *h) {
   constexpr int ND = 128;
   if (b.memD) return cudaSuccess;
   if (b.N <= 32) {
-    const size_t bfB = (size_t)t.nVoxPad * 3 * KF * sizeof(float);
-    const size_t kdB = (size_t)t.nSamPad * 3 * KF * sizeof(float);
-    b.bytesD = bfB + kdB + KF * KF * (sizeof(float) + sizeof(double));
-    cudaError_t e = cudaMalloc(&b.memD, b.bytesD);
-    if (e != cudaSuccess) { b.memD = nullptr; return e; }
-    b.facCol = (uint16_t *)b.memD;
-    b.facRow = (uint16_t *)((unsigned char *)b.memD + bfB);
-    b.Md = (float *)((unsigned char *)b.memD + bfB + kdB);
-    h->bytes += (int64_t)b.bytesD;
-    // voxel side of the reduced basis: fixed for the operator
-    e = tc_deriv_basis(h, b.facCol, b.Md, (double *)(b.Md + KF * KF), &b.rankD, &b.kfD);
+    // voxel side of the reduced basis: fixed for the operator; the tables are as wide
+    // as its rank asks for (96, 128 or 192 bytes a voxel and a sample)
+    const size_t nM = KF * KF, mB = nM * ((1 + tc_deriv_gram_blocks(h)) * sizeof(double) + sizeof(float));
+    cudaError_t e = cudaMalloc(&b.memM, mB);
+    if (e != cudaSuccess) { b.memM = nullptr; return e; }
+    double *Mv = (double *)b.memM;
+    b.Md = (float *)(Mv + nM * (1 + tc_deriv_gram_blocks(h)));
+    e = tc_deriv_basis(h, Mv + nM, b.Md, Mv, &b.rankD, &b.kfD);
     if (e == cudaSuccess && tc_configure_deriv(t.KP, b.N, b.kfD) < 1) e = cudaErrorInvalidConfiguration;
+    const size_t bfB = (size_t)t.nVoxPad * b.kfD * 4, kdB = (size_t)t.nSamPad * b.kfD * 4;
+    if (e == cudaSuccess && (e = cudaMalloc(&b.memD, bfB + kdB)) != cudaSuccess) b.memD = nullptr;
     if (e == cudaSuccess) {
+      b.facCol = (uint16_t *)b.memD;
+      b.facRow = (uint16_t *)((unsigned char *)b.memD + bfB);
+      e = tc_deriv_table(h, Mv, b.rankD, b.kfD, b.facCol);
+    }
+    if (e == cudaSuccess) {
+      b.bytesD = mB + bfB + kdB;
+      h->bytes += (int64_t)b.bytesD;
       b.fusedD = true;
     } else {
-      cudaFree(b.memD);
-      h->bytes -= (int64_t)b.bytesD;
-      b.memD = nullptr;
+      cudaFree(b.memM);
+      if (b.memD) cudaFree(b.memD);
+      b.memM = b.memD = nullptr;
       b.facCol = b.facRow = nullptr;
       b.Md = nullptr;
     }

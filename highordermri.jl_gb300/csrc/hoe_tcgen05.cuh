@@ -38,7 +38,8 @@ struct TcBuffers {
   float *Md = nullptr;      // reduced-basis rotation [KF x KF] of the one-pass path
   int rankD = 0, kfD = 48;  // its rank and the tables' 32-bit words a row (24, 32 or 48)
   bool fusedD = false;
-  void *memD = nullptr;
+  void *memM = nullptr;     // Md and what its making needs
+  void *memD = nullptr;     // the tables, or the B operand and slots
   size_t bytesD = 0;
   int gridD = 1, slotsD = 1;
 };
