@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_tc_backward(const __grid_cons
     auto seg_len = [&](int ch) { return min(min(BW_GROUP - ch % BW_GROUP, p.nChunks - ch), nIter - segBeg); };
     segEnd = seg_len(ch0);
     auto flush = [&]() {
-      const bool got = ok && wait_bar(segdone, seg, abort, p.err);
+      const bool got = ok && wait_bar_warp(segdone, seg, abort, p.err);
       tc_fence_after();
       if (got) {
 #pragma unroll
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_tc_backward(const __grid_cons
         }
       }
       if (!__all_sync(0xffffffffu, wready) &&
-          (!wait_bar(pfull + 8 * par, pr, abort, p.err) || !wait_bar(wfull + 8 * par, pr, abort, p.err))) {
+          (!wait_bar_warp(pfull + 8 * par, pr, abort, p.err) || !wait_bar_warp(wfull + 8 * par, pr, abort, p.err))) {
         ok = false;
         break;
       }
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_tc_backward(const __grid_cons
       if (it >= segEnd && __all_sync(0xffffffffu, mbar_test(segdone, seg))) flush();
       // G as BF16 hi/lo into the A tile of parity par, once the dk MMAs of
       // stage it-2 have read it
-      if (it >= 2 && !__all_sync(0xffffffffu, gready) && !wait_bar(gfree + 8 * par, pr ^ 1u, abort, p.err)) {
+      if (it >= 2 && !__all_sync(0xffffffffu, gready) && !wait_bar_warp(gfree + 8 * par, pr ^ 1u, abort, p.err)) {
         ok = false;
         break;
       }

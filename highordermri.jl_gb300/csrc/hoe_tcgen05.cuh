@@ -213,16 +213,26 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, uint32_t
   if (mbar_try_wait(bar, parity)) return true;
   return wait_bar_slow(bar, parity, abort, gerr, lim);
 }
-__device__ __forceinline__ bool wait_bar(uint64_t *bar, uint32_t parity, volatile int *abort,
-                                         int *gerr, uint64_t lim = 0) {
-  return wait_bar(smem_u32(bar), parity, smem_u32(const_cast<int *>(abort)), gerr, lim);
+// The same wait of a whole converged warp: the result is the same in all lanes (any
+// lane's failure counts) and the warp stays converged, as the tcgen05 loads and
+// stores that follow demand.  Its branches are uniform, which also saves registers.
+__device__ __noinline__ bool wait_warp_slow(uint32_t bar, uint32_t parity, uint32_t abort, int *gerr, uint64_t lim) {
+  const uint64_t t0 = globaltimer();
+  if (lim == 0) lim = kWaitNs;
+  for (;;) {
+    if (__all_sync(0xffffffffu, mbar_try_wait_sleep(bar, parity))) return true;
+    if (__any_sync(0xffffffffu, ld_shared_volatile(abort))) return false;
+    if (__any_sync(0xffffffffu, globaltimer() - t0 > lim)) {
+      st_shared_volatile(abort, 1);
+      atomicExch(gerr, HOE_ERR_TIMEOUT);
+      __syncwarp();
+      return false;
+    }
+  }
 }
-
-// Bounded wait made by every lane of a converged warp; the result is the same
-// in all lanes (any lane's failure counts), so the warp stays converged.
-template <class B, class A>
-__device__ __forceinline__ bool wait_bar_warp(B bar, uint32_t parity, A abort, int *gerr, uint64_t lim = 0) {
-  return __all_sync(0xffffffffu, wait_bar(bar, parity, abort, gerr, lim));
+__device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity, uint32_t abort, int *gerr, uint64_t lim = 0) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return wait_warp_slow(bar, parity, abort, gerr, lim);
 }
 
 // One lane of a converged warp (elect.sync).  MMA issuers run their loop with
