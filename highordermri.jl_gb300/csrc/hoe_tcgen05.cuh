@@ -143,10 +143,8 @@ __device__ __forceinline__ uint64_t globaltimer() {
   return t;
 }
 
-
-// Barriers are named by their shared-memory address (a 32-bit value) or by a
-// pointer; the address form saves the 64-bit arithmetic and the conversion in
-// loops that are short of issue slots.
+// Barriers are named by their shared-memory address (a 32-bit value), which saves
+// 64-bit arithmetic in loops that are short of issue slots.
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -254,30 +252,21 @@ __device__ __noinline__ bool drain_bar(uint32_t bar, uint32_t parity) {
     if (globaltimer() - t0 > kWaitNs) return false;
   return true;
 }
-__device__ __forceinline__ bool drain_bar(uint64_t *bar, uint32_t parity) { return drain_bar(smem_u32(bar), parity); }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) { mbar_arrive(smem_u32(bar)); }
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) { mbar_expect_tx(smem_u32(bar), bytes); }
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
       "l"(src), "r"(bytes), "r"(bar)
       : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-  bulk_g2s(smem_u32(dst), src, bytes, smem_u32(bar));
 }
 __device__ __forceinline__ void umma_tf32(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                           uint32_t accumulate) {
@@ -305,7 +294,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t *w) {
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint64_t *bar) { umma_commit(smem_u32(bar)); }
 __device__ __forceinline__ void tc_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
