@@ -51,7 +51,7 @@ def stored(t):
     """The tensor with its values in memory as they read: a lazy conjugate
     (x.conj()) or negation (x.conj().imag) is carried out, since the library gets
     the address of the values."""
-    return t.resolve_conj().resolve_neg()
+    return t.resolve_conj().resolve_neg() if t.is_conj() or t.is_neg() else t
 
 
 class ArgumentError(ValueError):

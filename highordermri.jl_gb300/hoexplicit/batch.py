@@ -15,6 +15,7 @@ import weakref
 
 from . import _lib
 from ._lib import ArgumentError, DimensionMismatch, stored
+from .operator import _direct
 from .recon import DEFAULT_ITERATIONS, DEFAULT_REL_TOL, STATUS, _device_vector
 
 
@@ -53,6 +54,9 @@ class OperatorBatch:
             raise DimensionMismatch(f"{name}: {len(vs)} vectors for {len(self.ops)} members")
         out = []
         for v, n, op in zip(vs, lens, self.ops):
+            if _direct(op, v, n):
+                out.append(v)
+                continue
             if not isinstance(v, torch.Tensor):
                 v = torch.from_numpy(v)
             if v.numel() != n:
