@@ -270,11 +270,10 @@ __global__ void k_tc_deriv_reduce(const float2 *__restrict__ part, int nSamPad, 
 
 // These kernels around the contraction are bound by their latency (3 to 5 us each
 // at any size up to 100x100): so no divisions by run-time values (64-bit ones took
-// half of the 257 instructions a warp of k_tc_adj_reduce), and what depends only on
-// the operator is read and worked out before pdl_wait.  With the contraction's early
-// start (pdl_wait in its loader): forward and adjoint at 32x32 / 1,000 samples / 4
-// coils 22.4 -> 19.2 us, 64x64 / 4,096 / 8 36.7 -> 35.2, 96x96 / 6,000 / 64 149 ->
-// 145, 200x200 / 12,000 / 16 508 -> 504.
+// half of k_tc_adj_reduce's instructions), and what depends only on the operator is
+// read and worked out before pdl_wait.  With the contraction's early start
+// (pdl_wait in its loader), forward and adjoint at 32x32 / 1,000 samples / 4 coils
+// take 19.2 us instead of 22.4, at 200x200 / 12,000 / 16 504 instead of 508.
 //
 // Adjoint reduction over the written slots: conj(csm), sum over coils,
 // scale, scatter into the full grid; the threads after the voxels' write
