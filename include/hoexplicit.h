@@ -234,6 +234,8 @@ HOE_API void hoe_free(hoe_handle *h);      /* closes if needed and frees the hos
 HOE_API int  hoe_is_closed(const hoe_handle *h);
 HOE_API const char *hoe_last_error(const hoe_handle *h);
 HOE_API int  hoe_get_info(const hoe_handle *h, hoe_info *out);
+/* Where this call or hoe_autotune prepares the tensor-core engine, it waits for the
+ * last hoe_set_kspha queued on any stream before it. */
 HOE_API int  hoe_set_engine(hoe_handle *h, int32_t engine);
 /* Tracing: with timing enabled, CUDA events are recorded on the call's stream
  * around each forward/adjoint and its main kernel; hoe_get_timings waits for
